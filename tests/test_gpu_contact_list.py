@@ -55,3 +55,19 @@ def test_rebuilt_lists_equal_the_oracles(cuda, oracle, n, spread, speed, orderin
         assert np.array_equal(gi[:, :m], ci[:, :m])
     if speed < 0 and n > 100:
         assert longest[-1] > longest[0]  # the list had to grow
+
+
+@pytest.mark.parametrize("per_particle", [False, True])
+@pytest.mark.parametrize("n,spread", [(2, 1.0), (257, 1.2), (1000, 1.7)])
+def test_hertz_force_against_the_oracle(cuda, oracle, n, spread, per_particle):
+    """Every operation behind the overlap is a rounding or two of a smooth
+    law: norm-wise within the contact bar of 1e-12 of the oracle."""
+    prob = _cloud(n, spread, per_particle, 0.0, 31 + n)
+    if n == 2:  # one overlapping pair
+        prob["x"][1] = prob["x"][0] + np.array([1.0e-3, 1.1e-3, -0.7e-3])
+    g, c = _pair(cuda, oracle, prob)
+    for s in (g, c):
+        s.compute_force()
+    a, b = g.get("f"), c.get("f")
+    assert np.linalg.norm(b) > 0.0
+    assert np.linalg.norm(a - b) <= 1e-12 * np.linalg.norm(b)
