@@ -1482,7 +1482,7 @@ static int launch_energy(cpd_system* s, const ParticleView& p, double* partials,
 static cpd_status sum_energy_partials(cpd_system* s, int rows, double* total_W, double* total_D)
 {
     CPD_CUDA(cudaGetLastError());
-    CPD_LAUNCHED(launch_sum_partials(s->red, rows, 2, s->red_out + 2, s->stream));
+    CPD_LAUNCHED(launch_sum_partials(s->red, rows, s->red_out + 2, s->stream));
     CPD_CUDA(cudaMemcpyAsync(s->h_red + 2, s->red_out + 2, sizeof(double) * 2,
                              cudaMemcpyDeviceToHost, s->stream));
     CPD_CUDA(cudaStreamSynchronize(s->stream));
@@ -2010,6 +2010,6 @@ extern "C" cpd_status cpd_compute_energy_noalloc(cpd_system* s, double* W_out,
     // nothing left in the scratch by an earlier call reaches the result.
     const int prows = launch_energy(s, p, scratch, nb, kNoAllocMaxBlocks);
     CPD_CUDA(cudaGetLastError());
-    CPD_LAUNCHED(launch_sum_partials(scratch, prows, 2, totals_out, s->stream));
+    CPD_LAUNCHED(launch_sum_partials(scratch, prows, totals_out, s->stream));
     return CPD_OK;
 }

@@ -255,8 +255,8 @@ int launch_prenotch(const ParticleView& p, const EllView& nl, const double* v1,
                     cudaStream_t st);
 int launch_pd_stress(const ParticleView& p, const EllView& nl, const Model& md, double* sigma,
                      cudaStream_t st);
-int launch_sum_partials(const double* partials, int nblocks, int ncols,
-                        double* out, cudaStream_t st);
+// Sums of n rows of two columns (partials is overwritten).
+int launch_sum_partials(double* partials, int n, double* out, cudaStream_t st);
 int launch_max_partials(const double* partials, int nblocks, double* out,
                         cudaStream_t st);
 int energy_blocks(int64_t nrows);
