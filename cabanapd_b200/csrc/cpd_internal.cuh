@@ -277,6 +277,16 @@ struct __align__(16) MixedStencil {
 struct __align__(32) MixedU {
     float4 hi, lo;
 };
+// A whole 32-byte gather record in one load (two 16-byte loads touch every line
+// of a warp's records twice).
+__device__ __forceinline__ double4 load_record(const double4* p)
+{
+    double4 v;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
+        : "l"(p));
+    return v;
+}
 struct MixedView {
     const float4* xh;  // positions, FP32 hi part
     const float4* xl;  // positions, FP32 lo part (x - hi)

@@ -1662,7 +1662,7 @@ namespace {
 cudaError_t lattice_cell_layout(const ParticleView& p, const double* h,
                                 const std::vector<MixedStencil>& tab, int64_t rows,
                                 MixedState& m, std::vector<unsigned int>& delta, int& launches,
-                                int& layout, cudaStream_t st)
+                                int& layout, int64_t* box, cudaStream_t st)
 {
     layout = 0;
     if (p.n <= 0 || rows <= 0) return cudaSuccess;
@@ -1703,6 +1703,7 @@ cudaError_t lattice_cell_layout(const ParticleView& p, const double* h,
         nc[d] = (int64_t)std::llround((from_bits(hb[3 + d]) - lo[d]) / h[d]) + 1;
     }
     const int64_t cells = nc[0] * nc[1] * nc[2];
+    for (int d = 0; d < 3; ++d) box[d] = nc[d];
     // A sparse outline would need too many empty records.
     if (cells > 4 * p.n + 4096 || cells >= ((int64_t)1 << 31)) return cudaSuccess;
     CPD_RET(dev_alloc(&buf.cell, sizeof(int32_t) * (size_t)p.npad, st));
@@ -1746,6 +1747,30 @@ cudaError_t lattice_cell_layout(const ParticleView& p, const double* h,
 #undef CPD_RET
 }  // namespace
 
+// Warps of a box of lattice lines in tile order: tiles of TY x TZ lines, one
+// chunk of 32 rows of each line after the other, so that the warps of a block
+// read overlapping lines in y and in z.
+static void box_tile_order(const int64_t* box, int64_t frozen, int64_t nw,
+                           std::vector<int32_t>& order)
+{
+    static const int TY = [] { const char* e = getenv("T_Y"); return e ? atoi(e) : 4; }();
+    static const int TZ = [] { const char* e = getenv("T_Z"); return e ? atoi(e) : 4; }();
+    const int64_t ty = (box[1] + TY - 1) / TY, tx = (box[0] + 31) / 32 + 1;
+    const int64_t tiles = ty * ((box[2] + TZ - 1) / TZ) * tx;
+    // Tile of each warp, by its first row; counting sort (stable: within a
+    // tile the warps stay in row order).
+    std::vector<int32_t> tile(nw), start(tiles + 1, 0);
+    for (int64_t q = 0; q < nw; ++q) {
+        const int64_t r = frozen + 32 * q, line = r / box[0];
+        const int64_t x = (r - line * box[0] + 16) / 32, y = line % box[1], z = line / box[1];
+        tile[q] = (int32_t)(x + tx * (y / TY + ty * (z / TZ)));
+        start[tile[q] + 1]++;
+    }
+    for (int64_t t = 0; t < tiles; ++t) start[t + 1] += start[t];
+    order.resize(nw);
+    for (int64_t q = 0; q < nw; ++q) order[start[tile[q]]++] = (int32_t)q;
+}
+
 int lattice_layout_probe(const ParticleView& p, const double* h, cudaStream_t st)
 {
     // The layout test alone: no table deltas are kept and the system's
@@ -1754,8 +1779,9 @@ int lattice_layout_probe(const ParticleView& p, const double* h, cudaStream_t st
     std::vector<MixedStencil> none;
     std::vector<unsigned int> delta;
     int launches = 0, layout = 0;
+    int64_t box[3];
     const cudaError_t e = lattice_cell_layout(p, h, none, p.n - p.frozen, probe, delta,
-                                              launches, layout, st);
+                                              launches, layout, box, st);
     if (probe.gcell) dev_free(probe.gcell, st);
     return e == cudaSuccess ? layout : 0;
 }
@@ -1902,8 +1928,10 @@ int prepare_mixed(const ParticleView& p, const NeighborList& pd, double cutoff, 
             // mask pass itself.
             int layout = 0;
             std::vector<unsigned int> delta(kDeltaSlots, 0xffffffffu);
+            int64_t box[3] = {0, 0, 0};
             if (lattice && !tab.empty())
-                CPD_TRY(lattice_cell_layout(p, h, tab, rows, m, delta, launches, layout, st));
+                CPD_TRY(lattice_cell_layout(p, h, tab, rows, m, delta, launches, layout, box,
+                                            st));
             if (fp32 && layout == 2) {
                 CPD_TRY(dev_free(m.gcell, st));
                 m.gcell = nullptr;
@@ -2032,19 +2060,27 @@ int prepare_mixed(const ParticleView& p, const NeighborList& pd, double cutoff, 
                     // Warp lists, each in the tile order of tile_chunk: warps
                     // of kinds 2 and 3 and the rest (the split mixed forms);
                     // warps of kinds 1-3 and of kind 0 (the stencil kernels).
-                    int g = 0;
-                    const EllView tv = tile_view(pd.view(), rows, kBlock, &g);
-                    const int64_t S = tv.stride, W = kBlock / 32;
-                    std::vector<int32_t> lean, rest, sten, irr;
+                    std::vector<int32_t> order, lean, rest, sten, irr;
+                    if (layout == 1 && box[0] >= 64) {
+                        box_tile_order(box, p.frozen, nw, order);
+                    } else {
+                        int g = 0;
+                        const EllView tv = tile_view(pd.view(), rows, kBlock, &g);
+                        const int64_t S = tv.stride, W = kBlock / 32;
+                        order.reserve(nw);
+                        for (int64_t b = 0; b < g; ++b)
+                            for (int64_t w = 0; w < W; ++w) {
+                                const int64_t q =
+                                    S > 1 ? (W * (b / S) + w) * S + b % S : W * b + w;
+                                if (q < nw) order.push_back((int32_t)q);
+                            }
+                    }
                     lean.reserve(nw);
                     sten.reserve(nw);
-                    for (int64_t b = 0; b < g; ++b)
-                        for (int64_t w = 0; w < W; ++w) {
-                            const int64_t q = S > 1 ? (W * (b / S) + w) * S + b % S : W * b + w;
-                            if (q >= nw) continue;
-                            (kinds[q] >= 2 ? lean : rest).push_back((int32_t)q);
-                            (kinds[q] >= 1 ? sten : irr).push_back((int32_t)q);
-                        }
+                    for (const int32_t q : order) {
+                        (kinds[q] >= 2 ? lean : rest).push_back(q);
+                        (kinds[q] >= 1 ? sten : irr).push_back(q);
+                    }
                     auto upload = [&](const std::vector<int32_t>& v, int32_t** dst,
                                       int64_t* count) -> bool {
                         *count = (int64_t)v.size();

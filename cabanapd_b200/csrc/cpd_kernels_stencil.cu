@@ -50,7 +50,28 @@
 namespace cpd {
 namespace {
 
-constexpr int kBlock = 256;
+#ifndef S64_BLOCK
+#define S64_BLOCK 512
+#endif
+#ifndef S64_MINB
+#define S64_MINB 2
+#endif
+#ifndef S64_PARTS
+#define S64_PARTS 1
+#endif
+#ifndef S32_MINB
+#define S32_MINB 2
+#endif
+#ifndef S32_SYNC
+#define S32_SYNC 0
+#endif
+#ifndef S64_SYNC
+#define S64_SYNC 0
+#endif
+#ifndef S64_EO
+#define S64_EO 0
+#endif
+constexpr int kBlock = S64_BLOCK;
 inline int blocks_for(int64_t rows) { return (int)((rows + kBlock - 1) / kBlock); }
 
 // High 32 bits of a double (host).
@@ -170,12 +191,24 @@ __device__ __forceinline__ void stencil_bond64(const StencilEntry64& e, const do
     const double hx = uj.x - ui.x, hy = uj.y - ui.y, hz = uj.z - ui.z;
     const double num = fma(hz, hz + e.tz, fma(hy, hy + e.ty, hx * (hx + e.tx)));
     const double q = num * e.ixi2;
+#if S64_EO
+    const double q2 = q * q;
+    double t = h[(NP - 1) & ~1], o = h[(NP - 2) | 1];
+#pragma unroll
+    for (int k = ((NP - 1) & ~1) - 2; k >= 0; k -= 2) t = fma(t, q2, h[k]);
+#pragma unroll
+    for (int k = ((NP - 2) | 1) - 2; k >= 1; k -= 2) o = fma(o, q2, h[k]);
+    t = fma(o, q, t);
+#else
     double t = h[NP - 1];
 #pragma unroll
     for (int k = NP - 2; k >= 0; --k) t = fma(t, q, h[k]);
+#endif
     double F = (num * e.K) * t;
     if (!UNIFORM) F *= uj.w;
-    const bool in = ((uint32_t)__double2hiint(num) & 0x7fffffffu) < e.khi;
+    // |num|'s high word below khi, compared as FP32 patterns, which order as
+    // the words do (one instruction, false for NaN).
+    const bool in = fabsf(__int_as_float(__double2hiint(num))) < __uint_as_float(e.khi);
     if (on && !in) pend |= bit;
     F = (on && in) ? F : 0.0;
     fx = fma(F, e.ex + hx, fx);
@@ -297,7 +330,7 @@ __device__ __forceinline__ void clear_bond_bit(const EllView& nl, const StencilR
 // TAB: the table's size (Stencil64 or Stencil64W); its bond-bit words NW.
 template <bool FRACTURE, bool UNIFORM, int K0, int K1, int NP, bool LAST, bool ENERGY = false,
           class TAB = Stencil64>
-__global__ void __launch_bounds__(kBlock, 4)
+__global__ void __launch_bounds__(kBlock, S64_MINB)
     k_pmb_stencil64(ParticleView p, EllView nl, StencilRows sr,
                     const double4* __restrict__ U4, double4* __restrict__ FPART,
                     StepEpilogue ep, const TAB st, const double* __restrict__ vol_sums,
@@ -346,8 +379,9 @@ __global__ void __launch_bounds__(kBlock, 4)
     for (int k = K0; k < K1; ++k) {
         const int w = k >> 5;
         const uint32_t bit = 1u << (k & 31);
+        if (S64_SYNC && k > K0 && (k % (S64_SYNC ? S64_SYNC : 1)) == 0) __syncthreads();
         const StencilEntry64& e = st.e[k];
-        const double4 uj = *reinterpret_cast<const double4*>(rb + e.boff);
+        const double4 uj = load_record(reinterpret_cast<const double4*>(rb + e.boff));
         stencil_bond64<UNIFORM, NP, ENERGY>(e, st.h, uj, ui, (ew[w] & bit) != 0u, bit, pend[w],
                                             fx, fy, fz, st.sh, ENERGY ? st.kw[k] : 0.0, &wsum);
     }
@@ -465,7 +499,7 @@ __device__ __forceinline__ void stencil_bond32(const StencilEntry32& e, const fl
 // force/CabanaPD_PMB.hpp:289-339), after this step's bond breaking; the
 // warp's sums of W_i vol_i and phi_i go to ep.energy_part.
 template <bool FRACTURE, bool UNIFORM, int NT, bool ENERGY = false>
-__global__ void __launch_bounds__(kBlock, 3)
+__global__ void __launch_bounds__(kBlock, S32_MINB)
     k_pmb_stencil32(ParticleView p, EllView nl, StencilRows sr, const MixedU* __restrict__ U2,
                     StepEpilogue ep, const Stencil32 st, const double* __restrict__ vol_sums)
 {
@@ -497,6 +531,7 @@ __global__ void __launch_bounds__(kBlock, 3)
     for (int k = 0; k < NT; ++k) {
         const int w = k >> 5;
         const uint32_t bit = 1u << (k & 31);
+        if (S32_SYNC && k > 0 && (k % (S32_SYNC ? S32_SYNC : 1)) == 0) __syncthreads();
         const StencilEntry32& e = st.e[k];
         const MixedU uj = *reinterpret_cast<const MixedU*>(rb + e.boff);
         stencil_bond32<UNIFORM, ENERGY>(e, st.h, uj, nh_xy, nh_z, nl_xy, nl_z,
@@ -843,10 +878,14 @@ int launch_pd_force_stencil64(const ParticleView& p, const EllView& nl, const Mo
         // row plate: 3.14 ms per step for the two, 3.30 ms for one walk).
 #define CPD_ST64X(F, U, NT, NP, E)                                                           \
     do {                                                                                     \
-        k_pmb_stencil64<F, U, 0, 64, NP, false, E><<<g, kBlock, 0, st>>>(                    \
+        if (S64_PARTS == 1) {                                                                 \
+        k_pmb_stencil64<F, U, 0, NT, NP, true, E><<<g, kBlock, 0, st>>>(                    \
+            p, nl, sr, m.u4, m.f64part, ep, S, m.vol_sums, m.gcell);                         \
+        } else { \
+    k_pmb_stencil64<F, U, 0, 64, NP, false, E><<<g, kBlock, 0, st>>>(                    \
             p, nl, sr, m.u4, m.f64part, ep, S, m.vol_sums, m.gcell);                         \
         k_pmb_stencil64<F, U, 64, NT, NP, true, E><<<g, kBlock, 0, st>>>(                    \
-            p, nl, sr, m.u4, m.f64part, ep, S, m.vol_sums, m.gcell);                         \
+            p, nl, sr, m.u4, m.f64part, ep, S, m.vol_sums, m.gcell);  }                       \
     } while (0)
 #define CPD_ST64(F, U, NT, NP) CPD_ST64X(F, U, NT, NP, false)
         // Unrolled forms: the 122-entry table of a cubic lattice at a
