@@ -1747,24 +1747,28 @@ cudaError_t lattice_cell_layout(const ParticleView& p, const double* h,
 #undef CPD_RET
 }  // namespace
 
-// Warps of a box of lattice lines in tile order: tiles of TY x TZ lines, one
-// chunk of 32 rows of each line after the other, so that the warps of a block
-// read overlapping lines in y and in z.
+// Warps of a box of lattice lines in tile order: tiles of 4 x 4 lines (y, z),
+// one chunk of 32 rows of each line after the other, so that the warps of a
+// block read overlapping lines in y and in z.
 static void box_tile_order(const int64_t* box, int64_t frozen, int64_t nw,
                            std::vector<int32_t>& order)
 {
-    static const int TY = [] { const char* e = getenv("T_Y"); return e ? atoi(e) : 4; }();
-    static const int TZ = [] { const char* e = getenv("T_Z"); return e ? atoi(e) : 4; }();
+    constexpr int64_t TY = 4, TZ = 4;
     const int64_t ty = (box[1] + TY - 1) / TY, tx = (box[0] + 31) / 32 + 1;
     const int64_t tiles = ty * ((box[2] + TZ - 1) / TZ) * tx;
     // Tile of each warp, by its first row; counting sort (stable: within a
     // tile the warps stay in row order).
     std::vector<int32_t> tile(nw), start(tiles + 1, 0);
+    const int64_t line = frozen / box[0];
+    int64_t x = frozen - line * box[0], y = line % box[1], z = line / box[1];
     for (int64_t q = 0; q < nw; ++q) {
-        const int64_t r = frozen + 32 * q, line = r / box[0];
-        const int64_t x = (r - line * box[0] + 16) / 32, y = line % box[1], z = line / box[1];
-        tile[q] = (int32_t)(x + tx * (y / TY + ty * (z / TZ)));
+        tile[q] = (int32_t)((x + 16) / 32 + tx * (y / TY + ty * (z / TZ)));
         start[tile[q] + 1]++;
+        for (x += 32; x >= box[0]; x -= box[0])
+            if (++y == box[1]) {
+                y = 0;
+                ++z;
+            }
     }
     for (int64_t t = 0; t < tiles; ++t) start[t + 1] += start[t];
     order.resize(nw);
@@ -2057,9 +2061,10 @@ int prepare_mixed(const ParticleView& p, const NeighborList& pd, double cutoff, 
                     }
                 }
                 {
-                    // Warp lists, each in the tile order of tile_chunk: warps
-                    // of kinds 2 and 3 and the rest (the split mixed forms);
-                    // warps of kinds 1-3 and of kind 0 (the stencil kernels).
+                    // Warp lists, each in the tile order of the box, or else of
+                    // tile_chunk: warps of kinds 2 and 3 and the rest (the split
+                    // mixed forms); warps of kinds 1-3 and of kind 0 (the stencil
+                    // kernels).
                     std::vector<int32_t> order, lean, rest, sten, irr;
                     if (layout == 1 && box[0] >= 64) {
                         box_tile_order(box, p.frozen, nw, order);
