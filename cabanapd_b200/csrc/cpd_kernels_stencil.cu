@@ -917,7 +917,7 @@ int launch_pd_force_stencil64(const ParticleView& p, const EllView& nl, const Mo
         }
 #undef CPD_ST64
 #undef CPD_ST64X
-        launched += 2;
+        launched += S64_PARTS;
     }
     if (m.nirregular > 0)
         launched += launch_pd_force_fast(p, nl, md, ep, st, m.irregular_list, m.nirregular);
