@@ -277,16 +277,11 @@ struct __align__(16) MixedStencil {
 struct __align__(32) MixedU {
     float4 hi, lo;
 };
-// A whole 32-byte gather record in one load (two 16-byte loads touch every line
-// of a warp's records twice).
-__device__ __forceinline__ double4 load_record(const double4* p)
-{
-    double4 v;
-    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-        : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
-        : "l"(p));
-    return v;
-}
+// An FP64 gather record (the layout of double4) that is read in one 32-byte
+// load.
+struct __align__(32) Record64 {
+    double x, y, z, w;
+};
 struct MixedView {
     const float4* xh;  // positions, FP32 hi part
     const float4* xl;  // positions, FP32 lo part (x - hi)
@@ -442,8 +437,8 @@ struct MixedState {
     // so i + delta of an absent stencil entry stays inside the allocation.
     Stencil64* st64 = nullptr;
     Stencil64W* st64w = nullptr;  // tables past kStencilMax entries
-    // The FP64 stencil walk runs in two launches: the first one's force sum
-    // per row (x, y, z; w unused), which the second one continues.
+    // Wide tables: the force sum per row (x, y, z; w: the energy sum) that
+    // one launch of the walk passes on to the next.
     double4* f64part = nullptr;
     // Lattice-cell layout of the FP64 gather records (a lattice body whose
     // particle order is not one box of lattice lines, e.g. with holes): row

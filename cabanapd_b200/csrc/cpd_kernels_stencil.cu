@@ -50,29 +50,14 @@
 namespace cpd {
 namespace {
 
-#ifndef S64_BLOCK
-#define S64_BLOCK 512
-#endif
-#ifndef S64_MINB
-#define S64_MINB 2
-#endif
-#ifndef S64_PARTS
-#define S64_PARTS 1
-#endif
-#ifndef S32_MINB
-#define S32_MINB 2
-#endif
-#ifndef S32_SYNC
-#define S32_SYNC 0
-#endif
-#ifndef S64_SYNC
-#define S64_SYNC 0
-#endif
-#ifndef S64_EO
-#define S64_EO 0
-#endif
-constexpr int kBlock = S64_BLOCK;
+constexpr int kBlock = 256;  // record packing
+// The table walks: 512 threads, two blocks per SM (64 registers a thread).
+constexpr int kWalkBlock = 512;
 inline int blocks_for(int64_t rows) { return (int)((rows + kBlock - 1) / kBlock); }
+inline int walk_blocks(int64_t warps)
+{
+    return (int)((warps + kWalkBlock / 32 - 1) / (kWalkBlock / 32));
+}
 
 // High 32 bits of a double (host).
 inline uint32_t hi_word(double v)
@@ -183,7 +168,7 @@ __device__ __forceinline__ bool exact_bond(const ParticleView& p, int64_t i, int
 // ENERGY: the bond's strain energy kw s^2 into w as well, s = q S(q).
 template <bool UNIFORM, int NP, bool ENERGY = false>
 __device__ __forceinline__ void stencil_bond64(const StencilEntry64& e, const double* h,
-                                               const double4& uj, const double4& ui, bool on,
+                                               const Record64& uj, const double4& ui, bool on,
                                                uint32_t bit, uint32_t& pend, double& fx,
                                                double& fy, double& fz, const double* sh = nullptr,
                                                double kw = 0.0, double* w = nullptr)
@@ -191,19 +176,9 @@ __device__ __forceinline__ void stencil_bond64(const StencilEntry64& e, const do
     const double hx = uj.x - ui.x, hy = uj.y - ui.y, hz = uj.z - ui.z;
     const double num = fma(hz, hz + e.tz, fma(hy, hy + e.ty, hx * (hx + e.tx)));
     const double q = num * e.ixi2;
-#if S64_EO
-    const double q2 = q * q;
-    double t = h[(NP - 1) & ~1], o = h[(NP - 2) | 1];
-#pragma unroll
-    for (int k = ((NP - 1) & ~1) - 2; k >= 0; k -= 2) t = fma(t, q2, h[k]);
-#pragma unroll
-    for (int k = ((NP - 2) | 1) - 2; k >= 1; k -= 2) o = fma(o, q2, h[k]);
-    t = fma(o, q, t);
-#else
     double t = h[NP - 1];
 #pragma unroll
     for (int k = NP - 2; k >= 0; --k) t = fma(t, q, h[k]);
-#endif
     double F = (num * e.K) * t;
     if (!UNIFORM) F *= uj.w;
     // |num|'s high word below khi, compared as FP32 patterns, which order as
@@ -317,11 +292,11 @@ __device__ __forceinline__ void clear_bond_bit(const EllView& nl, const StencilR
 // One warp per chunk of 32 rows of the stencil warp list; each row walks
 // table entries [K0, K1) (unrolled), and its own entries that are present
 // and intact are the bits of ew. NP: coefficients of the stretch
-// polynomial. The walk may be cut into parts launched one after the other
-// (the whole table's code exceeds the instruction cache): a part that does
-// not start at entry 0 continues from the partial force record FPART of the
-// previous part, and a part that is not the last stores its sum there;
-// the last part applies the step epilogue.
+// polynomial. Tables of up to 128 entries take one launch; the wide table is
+// cut into parts launched one after the other: a part that does not start at
+// entry 0 continues from the partial force record FPART of the previous part,
+// and a part that is not the last stores its sum there; the last part applies
+// the step epilogue. (FPART is not read or written by a single launch.)
 // ENERGY (output steps; one particle volume): the parts also sum the rows'
 // strain energy density W_i (the first part's in FPART's w), and the last
 // part writes W_i and phi_i = 1 - vol_sums[intact] / vol_sums[bonds] after
@@ -330,7 +305,7 @@ __device__ __forceinline__ void clear_bond_bit(const EllView& nl, const StencilR
 // TAB: the table's size (Stencil64 or Stencil64W); its bond-bit words NW.
 template <bool FRACTURE, bool UNIFORM, int K0, int K1, int NP, bool LAST, bool ENERGY = false,
           class TAB = Stencil64>
-__global__ void __launch_bounds__(kBlock, S64_MINB)
+__global__ void __launch_bounds__(kWalkBlock, 2)
     k_pmb_stencil64(ParticleView p, EllView nl, StencilRows sr,
                     const double4* __restrict__ U4, double4* __restrict__ FPART,
                     StepEpilogue ep, const TAB st, const double* __restrict__ vol_sums,
@@ -339,7 +314,7 @@ __global__ void __launch_bounds__(kBlock, S64_MINB)
     constexpr int NW = (int)(sizeof(st.e) / sizeof(st.e[0])) / 32;
     constexpr bool SUMS = ENERGY && LAST;
     const int lane = threadIdx.x & 31;
-    const int64_t slot = (int64_t)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
+    const int64_t slot = (int64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
     if (slot >= sr.wcount) return;
     const int64_t warp = sr.wlist[slot];
     const int64_t i = p.frozen + 32 * warp + lane;
@@ -369,19 +344,15 @@ __global__ void __launch_bounds__(kBlock, S64_MINB)
     // Fully unrolled, every entry of the range for every row: an absent entry
     // (no bit in ew) reads the record at i + delta_k (a neighbour, or a zero
     // guard record) and adds nothing, which costs less than a branch per
-    // entry. Entries past ntab are zero-filled and add nothing either. (A
-    // loop over chunks of 8 entries with the table in shared memory keeps
-    // the code inside the instruction cache but waits on the shared-memory
-    // loads: 4.75 vs 3.25 ms per step on the full plate; two rows per thread
-    // halves the instruction fetch per bond but needs 128 registers, and
-    // at 2 blocks per SM: 3.76 ms.)
+    // entry. Entries past ntab are zero-filled and add nothing either. The
+    // record is one 32-byte load (two 16-byte loads touch every line of a
+    // warp's records twice: 2.75 vs 2.51 ms per step on the 11.52 M plate).
 #pragma unroll
     for (int k = K0; k < K1; ++k) {
         const int w = k >> 5;
         const uint32_t bit = 1u << (k & 31);
-        if (S64_SYNC && k > K0 && (k % (S64_SYNC ? S64_SYNC : 1)) == 0) __syncthreads();
         const StencilEntry64& e = st.e[k];
-        const double4 uj = load_record(reinterpret_cast<const double4*>(rb + e.boff));
+        const Record64 uj = *reinterpret_cast<const Record64*>(rb + e.boff);
         stencil_bond64<UNIFORM, NP, ENERGY>(e, st.h, uj, ui, (ew[w] & bit) != 0u, bit, pend[w],
                                             fx, fy, fz, st.sh, ENERGY ? st.kw[k] : 0.0, &wsum);
     }
@@ -499,12 +470,12 @@ __device__ __forceinline__ void stencil_bond32(const StencilEntry32& e, const fl
 // force/CabanaPD_PMB.hpp:289-339), after this step's bond breaking; the
 // warp's sums of W_i vol_i and phi_i go to ep.energy_part.
 template <bool FRACTURE, bool UNIFORM, int NT, bool ENERGY = false>
-__global__ void __launch_bounds__(kBlock, S32_MINB)
+__global__ void __launch_bounds__(kWalkBlock, 2)
     k_pmb_stencil32(ParticleView p, EllView nl, StencilRows sr, const MixedU* __restrict__ U2,
                     StepEpilogue ep, const Stencil32 st, const double* __restrict__ vol_sums)
 {
     const int lane = threadIdx.x & 31;
-    const int64_t slot = (int64_t)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
+    const int64_t slot = (int64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
     if (slot >= sr.wcount) return;
     const int64_t warp = sr.wlist[slot];
     const int64_t i = p.frozen + 32 * warp + lane;
@@ -531,7 +502,6 @@ __global__ void __launch_bounds__(kBlock, S32_MINB)
     for (int k = 0; k < NT; ++k) {
         const int w = k >> 5;
         const uint32_t bit = 1u << (k & 31);
-        if (S32_SYNC && k > 0 && (k % (S32_SYNC ? S32_SYNC : 1)) == 0) __syncthreads();
         const StencilEntry32& e = st.e[k];
         const MixedU uj = *reinterpret_cast<const MixedU*>(rb + e.boff);
         stencil_bond32<UNIFORM, ENERGY>(e, st.h, uj, nh_xy, nh_z, nl_xy, nl_z,
@@ -777,7 +747,7 @@ int launch_pd_force_stencil32(const ParticleView& p, const EllView& nl, const Mo
 {
     if (p.n - p.frozen <= 0 || m.nstencil <= 0) return 0;
     const StencilRows sr{m.warp_kind, m.pmask, m.stencil_list, m.nstencil};
-    const int g = (int)((m.nstencil + kBlock / 32 - 1) / (kBlock / 32));
+    const int g = walk_blocks(m.nstencil);
     const bool uniform = m.vol_sums != nullptr;
     const Stencil32& S = *m.st32;
     const bool t122 = S.ntab == 122;
@@ -785,7 +755,7 @@ int launch_pd_force_stencil32(const ParticleView& p, const EllView& nl, const Mo
         // Output step: the energy forms (one particle volume only).
         if (!uniform) return -1;
 #define CPD_ST32E(F, NT) \
-    k_pmb_stencil32<F, true, NT, true><<<g, kBlock, 0, st>>>(p, nl, sr, m.u2, ep, S, m.vol_sums)
+    k_pmb_stencil32<F, true, NT, true><<<g, kWalkBlock, 0, st>>>(p, nl, sr, m.u2, ep, S, m.vol_sums)
         if (md.fracture) {
             if (t122) CPD_ST32E(true, 122); else CPD_ST32E(true, 128);
         } else {
@@ -795,7 +765,7 @@ int launch_pd_force_stencil32(const ParticleView& p, const EllView& nl, const Mo
         return 1;
     }
 #define CPD_ST32(F, U, NT) \
-    k_pmb_stencil32<F, U, NT><<<g, kBlock, 0, st>>>(p, nl, sr, m.u2, ep, S, nullptr)
+    k_pmb_stencil32<F, U, NT><<<g, kWalkBlock, 0, st>>>(p, nl, sr, m.u2, ep, S, nullptr)
     if (!uniform) {
         if (md.fracture) CPD_ST32(true, false, 128); else CPD_ST32(false, false, 128);
     } else if (md.fracture) {
@@ -823,7 +793,7 @@ int launch_pd_force_stencil64(const ParticleView& p, const EllView& nl, const Mo
     int launched = 0;
     if (m.nstencil > 0) {
         const StencilRows sr{m.warp_kind, m.pmask, m.stencil_list, m.nstencil};
-        const int g = (int)((m.nstencil + kBlock / 32 - 1) / (kBlock / 32));
+        const int g = walk_blocks(m.nstencil);
         const bool uniform = m.vol_sums != nullptr;
         if (m.st64w) {
             // Tables past 128 entries (a horizon of 4 spacings: 256): four
@@ -836,19 +806,19 @@ int launch_pd_force_stencil64(const ParticleView& p, const EllView& nl, const Mo
 #define CPD_ST64W(F, NP, E)                                                                   \
     do {                                                                                      \
         k_pmb_stencil64<F, true, 0, 64, NP, false, E, Stencil64W>                             \
-            <<<g, kBlock, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums, m.gcell);   \
+            <<<g, kWalkBlock, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums, m.gcell);   \
         k_pmb_stencil64<F, true, 64, 128, NP, false, E, Stencil64W>                           \
-            <<<g, kBlock, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums, m.gcell);   \
+            <<<g, kWalkBlock, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums, m.gcell);   \
         if (t192) {                                                                           \
             k_pmb_stencil64<F, true, 128, 192, NP, true, E, Stencil64W>                       \
-                <<<g, kBlock, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums,         \
+                <<<g, kWalkBlock, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums,         \
                                        m.gcell);                                              \
         } else {                                                                              \
             k_pmb_stencil64<F, true, 128, 192, NP, false, E, Stencil64W>                      \
-                <<<g, kBlock, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums,         \
+                <<<g, kWalkBlock, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums,         \
                                        m.gcell);                                              \
             k_pmb_stencil64<F, true, 192, 256, NP, true, E, Stencil64W>                       \
-                <<<g, kBlock, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums,         \
+                <<<g, kWalkBlock, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums,         \
                                        m.gcell);                                              \
         }                                                                                     \
     } while (0)
@@ -871,22 +841,9 @@ int launch_pd_force_stencil64(const ParticleView& p, const EllView& nl, const Mo
             return launched;
         }
         const Stencil64& S = *m.st64;
-        // Two launches over the table's halves (entries 0-63, then 64 on):
-        // the first stores its partial force and broken count per row, the
-        // second adds its own and runs the epilogue. Each is a shorter
-        // unrolled walk that stays in the instruction cache (B200, 11.52 M
-        // row plate: 3.14 ms per step for the two, 3.30 ms for one walk).
-#define CPD_ST64X(F, U, NT, NP, E)                                                           \
-    do {                                                                                     \
-        if (S64_PARTS == 1) {                                                                 \
-        k_pmb_stencil64<F, U, 0, NT, NP, true, E><<<g, kBlock, 0, st>>>(                    \
-            p, nl, sr, m.u4, m.f64part, ep, S, m.vol_sums, m.gcell);                         \
-        } else { \
-    k_pmb_stencil64<F, U, 0, 64, NP, false, E><<<g, kBlock, 0, st>>>(                    \
-            p, nl, sr, m.u4, m.f64part, ep, S, m.vol_sums, m.gcell);                         \
-        k_pmb_stencil64<F, U, 64, NT, NP, true, E><<<g, kBlock, 0, st>>>(                    \
-            p, nl, sr, m.u4, m.f64part, ep, S, m.vol_sums, m.gcell);  }                       \
-    } while (0)
+#define CPD_ST64X(F, U, NT, NP, E)                                       \
+    k_pmb_stencil64<F, U, 0, NT, NP, true, E><<<g, kWalkBlock, 0, st>>>( \
+        p, nl, sr, m.u4, nullptr, ep, S, m.vol_sums, m.gcell)
 #define CPD_ST64(F, U, NT, NP) CPD_ST64X(F, U, NT, NP, false)
         // Unrolled forms: the 122-entry table of a cubic lattice at a
         // 3.01-spacing horizon, else 128 entries (zero past ntab).
@@ -917,7 +874,7 @@ int launch_pd_force_stencil64(const ParticleView& p, const EllView& nl, const Mo
         }
 #undef CPD_ST64
 #undef CPD_ST64X
-        launched += S64_PARTS;
+        launched += 1;
     }
     if (m.nirregular > 0)
         launched += launch_pd_force_fast(p, nl, md, ep, st, m.irregular_list, m.nirregular);
