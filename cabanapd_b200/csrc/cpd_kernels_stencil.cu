@@ -672,9 +672,10 @@ bool prepare_stencil64(const ParticleView& p, const Model& md, const double* h,
     m.guard = G + 32;
     // Records by lattice cell (m.gcell) or by row.
     const size_t recs = (size_t)((m.gcell ? m.grid_cells : p.npad) + 2 * m.guard);
+    const size_t part_bytes = m.st64w ? sizeof(double4) * (size_t)p.npad : 0;
     if (dev_alloc(&m.u4_base, sizeof(double4) * recs, st) != cudaSuccess ||
         dev_alloc(&m.u4_alt_base, sizeof(double4) * recs, st) != cudaSuccess ||
-        dev_alloc(&m.f64part, sizeof(double4) * (size_t)p.npad, st) != cudaSuccess ||
+        (part_bytes > 0 && dev_alloc(&m.f64part, part_bytes, st) != cudaSuccess) ||
         cudaMemsetAsync(m.u4_base, 0, sizeof(double4) * recs, st) != cudaSuccess ||
         cudaMemsetAsync(m.u4_alt_base, 0, sizeof(double4) * recs, st) != cudaSuccess) {
         err = std::string("stencil gather records: ") + cudaGetErrorString(cudaGetLastError());
@@ -683,7 +684,7 @@ bool prepare_stencil64(const ParticleView& p, const Model& md, const double* h,
     }
     m.u4 = m.u4_base + m.guard;
     m.u4_alt = m.u4_alt_base + m.guard;
-    m.bytes += 2 * sizeof(double4) * recs + sizeof(double4) * (size_t)p.npad;
+    m.bytes += 2 * sizeof(double4) * recs + part_bytes;
     return true;
 }
 

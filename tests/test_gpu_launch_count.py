@@ -1,4 +1,7 @@
-"""cpd_kernel_launches of a step on the lattice-stencil kernels, exactly."""
+"""cpd_kernel_launches of a step on the lattice-stencil kernels, exactly, and
+the device bytes that the FP64 tables hold."""
+import ctypes
+
 import pytest
 
 from cabanapd_b200 import problems as P
@@ -29,3 +32,23 @@ def test_launches_of_a_step(precision, horizon_factor, entries, before, per_step
         s.step(steps)
         assert s.kernel_launches() - counted == before + per_step * steps
 
+
+def _bytes(system):
+    system.step(1)
+    n = ctypes.c_uint64()
+    assert system._lib.cpd_device_bytes(system._h, ctypes.byref(n)) == 0
+    return n.value
+
+
+@pytest.mark.parametrize("horizon_factor,layers,parts", [(3.01, 3, 0), (4.0, 4, 1)])
+def test_partial_forces_are_held_for_wide_tables_only(horizon_factor, layers, parts):
+    """Beyond the exact path's: the second displacement (24 bytes a row), two
+    buffers of 32-byte records with guards of the farthest offset, presence
+    masks of 4 bytes per 32 entries, lists and masks per warp (under 4 bytes a
+    row), and 32 bytes a row of partial forces where the walk has parts."""
+    rows = CELLS[0] * CELLS[1] * CELLS[2]
+    records = rows + 2 * (layers * CELLS[0] * CELLS[1] + 32)
+    masks = 16 if horizon_factor < 4 else 32
+    least = (24 + masks + 32 * parts) * rows + 64 * records
+    held = _bytes(_system(1, horizon_factor)) - _bytes(_system(0, horizon_factor))
+    assert least <= held <= least + 8 * rows
