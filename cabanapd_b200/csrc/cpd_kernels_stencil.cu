@@ -51,12 +51,36 @@ namespace cpd {
 namespace {
 
 constexpr int kBlock = 256;  // record packing
-// The table walks: 512 threads, two blocks per SM (64 registers a thread).
-constexpr int kWalkBlock = 512;
 inline int blocks_for(int64_t rows) { return (int)((rows + kBlock - 1) / kBlock); }
-inline int walk_blocks(int64_t warps)
+
+// The table walks take 512 threads a block, two blocks per SM (64 registers a
+// thread): the warps of a block walk the same code together, which the
+// instruction cache holds only in part (11.52 M plate, FP64: 2.51 vs 2.98 ms
+// per step in blocks of 256; FP32: 1.93 vs 2.26). A small body fills fewer SMs
+// that way, or one of them twice over, and its time is the busiest SM's: it
+// takes blocks of 256 where that SM then has less than `share` of the rows it
+// has in blocks of 512. Per step in blocks of 256 / 512 (cubes of 8, 33, 79,
+// 97, 157 and 176 thousand rows; the busiest SM's rows in ratio 1/2, 1/2, 3/4,
+// 3/4, 5/6, 5/6):
+//   FP64 19 / 23, 19 / 23, 35 / 40, 35 / 41, 58 / 58, 59 / 57 us: share 0.8;
+//   FP32 15 / 19, 15 / 20, 27 / 31, 27 / 31, 40 / 44, 41 / 45 us, and at 238
+//   (7/8) 58 / 58: share 0.875;
+// and between, where the ratio is one (43 to 74, 125 and 149 thousand), FP64
+// 25 / 23, 44 / 41, FP32 20 / 19, 39 / 31 us. The four launches of the wide
+// table gain from whole blocks sooner (20 thousand rows 72 / 83 us, 80 thousand,
+// ratio 3/4, 131 / 125): share 0.6.
+constexpr int kWalkBlock = 512, kSmallWalkBlock = 256;
+constexpr double kShare64 = 0.8, kShare64Wide = 0.6, kShare32 = 0.875;
+inline int walk_blocks(int64_t warps, int block)
 {
-    return (int)((warps + kWalkBlock / 32 - 1) / (kWalkBlock / 32));
+    return (int)((warps + block / 32 - 1) / (block / 32));
+}
+inline int walk_block(int64_t warps, double share)
+{
+    auto busiest = [&](int block) {
+        return (double)((walk_blocks(warps, block) + 147) / 148 * block);
+    };
+    return busiest(kSmallWalkBlock) < share * busiest(kWalkBlock) ? kSmallWalkBlock : kWalkBlock;
 }
 
 // High 32 bits of a double (host).
@@ -469,8 +493,13 @@ __device__ __forceinline__ void stencil_bond32(const StencilEntry32& e, const fl
 // / vol_sums[bonds] (the ordered FP64 sums of the damage formula,
 // force/CabanaPD_PMB.hpp:289-339), after this step's bond breaking; the
 // warp's sums of W_i vol_i and phi_i go to ep.energy_part.
-template <bool FRACTURE, bool UNIFORM, int NT, bool ENERGY = false>
-__global__ void __launch_bounds__(kWalkBlock, 2)
+// BLOCK, PER_SM: the launch bounds, 512 threads twice (64 registers) or 256
+// three times (80). Small bodies take the second: at one warp or two per
+// scheduler the spills of 64 registers are in the open (33 thousand rows 14.7
+// vs 16.5 us per step, both in blocks of 256).
+template <bool FRACTURE, bool UNIFORM, int NT, bool ENERGY = false, int BLOCK = kWalkBlock,
+          int PER_SM = 2>
+__global__ void __launch_bounds__(BLOCK, PER_SM)
     k_pmb_stencil32(ParticleView p, EllView nl, StencilRows sr, const MixedU* __restrict__ U2,
                     StepEpilogue ep, const Stencil32 st, const double* __restrict__ vol_sums)
 {
@@ -748,7 +777,8 @@ int launch_pd_force_stencil32(const ParticleView& p, const EllView& nl, const Mo
 {
     if (p.n - p.frozen <= 0 || m.nstencil <= 0) return 0;
     const StencilRows sr{m.warp_kind, m.pmask, m.stencil_list, m.nstencil};
-    const int g = walk_blocks(m.nstencil);
+    const int block = walk_block(m.nstencil, kShare32);
+    const int g = walk_blocks(m.nstencil, block);
     const bool uniform = m.vol_sums != nullptr;
     const Stencil32& S = *m.st32;
     const bool t122 = S.ntab == 122;
@@ -756,7 +786,7 @@ int launch_pd_force_stencil32(const ParticleView& p, const EllView& nl, const Mo
         // Output step: the energy forms (one particle volume only).
         if (!uniform) return -1;
 #define CPD_ST32E(F, NT) \
-    k_pmb_stencil32<F, true, NT, true><<<g, kWalkBlock, 0, st>>>(p, nl, sr, m.u2, ep, S, m.vol_sums)
+    k_pmb_stencil32<F, true, NT, true><<<g, block, 0, st>>>(p, nl, sr, m.u2, ep, S, m.vol_sums)
         if (md.fracture) {
             if (t122) CPD_ST32E(true, 122); else CPD_ST32E(true, 128);
         } else {
@@ -765,8 +795,15 @@ int launch_pd_force_stencil32(const ParticleView& p, const EllView& nl, const Mo
 #undef CPD_ST32E
         return 1;
     }
-#define CPD_ST32(F, U, NT) \
-    k_pmb_stencil32<F, U, NT><<<g, kWalkBlock, 0, st>>>(p, nl, sr, m.u2, ep, S, nullptr)
+#define CPD_ST32(F, U, NT)                                                           \
+    do {                                                                             \
+        if (block == kWalkBlock)                                                     \
+            k_pmb_stencil32<F, U, NT><<<g, block, 0, st>>>(p, nl, sr, m.u2, ep, S,   \
+                                                           nullptr);                 \
+        else                                                                         \
+            k_pmb_stencil32<F, U, NT, false, kSmallWalkBlock, 3>                     \
+                <<<g, block, 0, st>>>(p, nl, sr, m.u2, ep, S, nullptr);              \
+    } while (0)
     if (!uniform) {
         if (md.fracture) CPD_ST32(true, false, 128); else CPD_ST32(false, false, 128);
     } else if (md.fracture) {
@@ -794,7 +831,8 @@ int launch_pd_force_stencil64(const ParticleView& p, const EllView& nl, const Mo
     int launched = 0;
     if (m.nstencil > 0) {
         const StencilRows sr{m.warp_kind, m.pmask, m.stencil_list, m.nstencil};
-        const int g = walk_blocks(m.nstencil);
+        const int block = walk_block(m.nstencil, m.st64w ? kShare64Wide : kShare64);
+        const int g = walk_blocks(m.nstencil, block);
         const bool uniform = m.vol_sums != nullptr;
         if (m.st64w) {
             // Tables past 128 entries (a horizon of 4 spacings: 256): four
@@ -807,19 +845,19 @@ int launch_pd_force_stencil64(const ParticleView& p, const EllView& nl, const Mo
 #define CPD_ST64W(F, NP, E)                                                                   \
     do {                                                                                      \
         k_pmb_stencil64<F, true, 0, 64, NP, false, E, Stencil64W>                             \
-            <<<g, kWalkBlock, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums, m.gcell);   \
+            <<<g, block, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums, m.gcell);   \
         k_pmb_stencil64<F, true, 64, 128, NP, false, E, Stencil64W>                           \
-            <<<g, kWalkBlock, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums, m.gcell);   \
+            <<<g, block, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums, m.gcell);   \
         if (t192) {                                                                           \
             k_pmb_stencil64<F, true, 128, 192, NP, true, E, Stencil64W>                       \
-                <<<g, kWalkBlock, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums,         \
+                <<<g, block, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums,         \
                                        m.gcell);                                              \
         } else {                                                                              \
             k_pmb_stencil64<F, true, 128, 192, NP, false, E, Stencil64W>                      \
-                <<<g, kWalkBlock, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums,         \
+                <<<g, block, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums,         \
                                        m.gcell);                                              \
             k_pmb_stencil64<F, true, 192, 256, NP, true, E, Stencil64W>                       \
-                <<<g, kWalkBlock, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums,         \
+                <<<g, block, 0, st>>>(p, nl, sr, m.u4, m.f64part, ep, W, m.vol_sums,         \
                                        m.gcell);                                              \
         }                                                                                     \
     } while (0)
@@ -843,7 +881,7 @@ int launch_pd_force_stencil64(const ParticleView& p, const EllView& nl, const Mo
         }
         const Stencil64& S = *m.st64;
 #define CPD_ST64X(F, U, NT, NP, E)                                       \
-    k_pmb_stencil64<F, U, 0, NT, NP, true, E><<<g, kWalkBlock, 0, st>>>( \
+    k_pmb_stencil64<F, U, 0, NT, NP, true, E><<<g, block, 0, st>>>( \
         p, nl, sr, m.u4, nullptr, ep, S, m.vol_sums, m.gcell)
 #define CPD_ST64(F, U, NT, NP) CPD_ST64X(F, U, NT, NP, false)
         // Unrolled forms: the 122-entry table of a cubic lattice at a
