@@ -1749,7 +1749,15 @@ cudaError_t lattice_cell_layout(const ParticleView& p, const double* h,
 
 // Warps of a box of lattice lines in tile order: tiles of 4 x 4 lines (y, z),
 // one chunk of 32 rows of each line after the other, so that the warps of a
-// block read overlapping lines in y and in z.
+// block read overlapping lines in y and in z. Taken for planes of kTilePlane
+// rows on: the seven planes that rows at a three-spacing horizon read are then
+// 54 MB of records, and lines read from one plane leave the L2 before the next
+// plane's rows want them (FP32 walk, plates of nx x nx / 2 x 20, tile order
+// against tile_chunk's: 832 wide 1.18 vs 1.23 ms per step, 736 0.92 vs 0.95;
+// 640 0.706 vs 0.705, 512 0.460 vs 0.455, 256 x 128 x 8 0.072 vs 0.065; LPS
+// box of 1000 x 400 x 20 4.47 vs 4.61; the FP64 walk, bound by its arithmetic,
+// within 2% either way).
+constexpr int64_t kTilePlane = 240000;
 static void box_tile_order(const int64_t* box, int64_t frozen, int64_t nw,
                            std::vector<int32_t>& order)
 {
@@ -2061,12 +2069,12 @@ int prepare_mixed(const ParticleView& p, const NeighborList& pd, double cutoff, 
                     }
                 }
                 {
-                    // Warp lists, each in the tile order of the box, or else of
-                    // tile_chunk: warps of kinds 2 and 3 and the rest (the split
-                    // mixed forms); warps of kinds 1-3 and of kind 0 (the stencil
-                    // kernels).
+                    // Warp lists, each in the tile order of the box (large
+                    // planes) or of tile_chunk: warps of kinds 2 and 3 and the
+                    // rest (the split mixed forms); warps of kinds 1-3 and of
+                    // kind 0 (the stencil kernels).
                     std::vector<int32_t> order, lean, rest, sten, irr;
-                    if (layout == 1 && box[0] >= 64) {
+                    if (layout == 1 && box[0] >= 64 && box[0] * box[1] >= kTilePlane) {
                         box_tile_order(box, p.frozen, nw, order);
                     } else {
                         int g = 0;

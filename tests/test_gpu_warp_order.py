@@ -12,20 +12,23 @@ from cabanapd_b200 import problems as P
 
 pytestmark = pytest.mark.gpu
 
+STEPS = 4
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def _plate(cells, frozen=0):
     nx, ny, nz = cells
-    prob = P.plate_impact(num_cells=cells, steps=20, v0=60.0,
+    prob = P.plate_impact(num_cells=cells, steps=STEPS, v0=60.0,
                           size=(0.2, 0.2 * ny / nx, 0.2 * nz / nx))
     prob["n_frozen"] = frozen
     return prob
 
 
-@pytest.mark.parametrize("cells,frozen", [((64, 4, 4), 0), ((65, 9, 6), 0), ((97, 13, 7), 0),
-                                          ((128, 5, 3), 0), ((97, 13, 7), 97 * 3 + 40),
-                                          ((66, 11, 5), 33)])
+# (Planes of 240 thousand rows on are walked in tiles of 4 x 4 lines.)
+@pytest.mark.parametrize("cells,frozen", [((97, 13, 7), 97 * 3 + 40), ((600, 399, 2), 0),
+                                          ((600, 400, 2), 0), ((613, 397, 5), 0),
+                                          ((613, 393, 3), 613 * 3 + 40)])
 def test_every_row_is_advanced(oracle, cells, frozen):
     """A warp left out or taken twice leaves whole rows off by their own size;
     the FP64 path's bar is 1e-12 norm-wise."""
@@ -37,8 +40,8 @@ def test_every_row_is_advanced(oracle, cells, frozen):
         P.setup(s, prob)
     warps, irregular, _ = g.stencil_stats()
     assert warps + irregular == (len(prob["x"]) - frozen + 31) // 32
-    g.run(20)
-    o.run(20)
+    g.run(STEPS)
+    o.run(STEPS)
     for name in ("u", "v", "f"):
         a, b = g.get(name), o.get(name)
         assert np.linalg.norm(a - b) <= 1e-12 * np.linalg.norm(b), name
@@ -49,14 +52,14 @@ import sys
 sys.path.insert(0, sys.argv[1])
 import cabanapd_b200
 from cabanapd_b200 import problems as P
-prob = P.plate_impact(num_cells=(96, 48, 8), steps=20, v0=60.0, size=(0.2, 0.1, 0.2 * 8 / 96))
+prob = P.plate_impact(num_cells=(600, 405, 4), steps=3, v0=60.0, size=(0.2, 0.135, 0.2 * 4 / 600))
 s = cabanapd_b200.System(dict(prob["params"], precision=2))
 P.setup(s, prob)
-print(" ".join(v.hex() for v in s.step_energy(20)))
+print(" ".join(v.hex() for v in s.step_energy(3)))
 """
 
 
-@pytest.mark.parametrize("value", ["1", "0", "-3", "x"])
+@pytest.mark.parametrize("value", ["1", "x"])
 def test_totals_do_not_depend_on_the_callers_environment(value):
     """The order of the warps is the order of the energy partials, so the
     totals' last bits show it."""
