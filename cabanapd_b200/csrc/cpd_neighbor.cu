@@ -213,9 +213,15 @@ __global__ void __launch_bounds__(kBlock)
 // build left: rows of up to cap neighbours are complete and sorted by the
 // neighbours' caller index (user_id, or the index itself); when the longest
 // row (stats[0]) is longer, the caller takes k_fill on a longer list instead.
-// Rows are short here (contact lists), so they are sorted in place. One walk
-// over the cells instead of two: 0.47 ms for 4.0 M spheres with six contacts
-// each, 0.78 + 0.72 ms by count and fill on gathered positions.
+// Rows are sorted in place, so the list has at most kRefillRow columns. One
+// walk over the cells instead of two: 0.47 ms for 4.0 M spheres with six
+// contacts each, 0.78 + 0.72 ms by count and fill. Longer rows are k_fill's,
+// which sorts them in local memory: per step with a rebuild, 100 thousand
+// random points with rows of up to 23, 30, 46 and 78: 0.27, 0.36, 0.74 and 2.10
+// ms in one pass, 0.26, 0.32, 0.52 and 1.02 by count and fill, in cells of the
+// cutoff; 1.0 M points with rows of up to 24, 32 and 46: 1.25, 1.83 and 4.21
+// against 1.56, 2.14 and 3.97.
+constexpr int32_t kRefillRow = 32;
 __global__ void __launch_bounds__(kBlock)
     k_refill(const double* pos, int64_t n, int64_t npad, int64_t begin, Grid g,
              const int32_t* cell_start, CellOrder co, double rsqr, int32_t* count,
@@ -523,8 +529,9 @@ int build_neighbor_list(const double* x, const double* disp, int64_t n, int64_t 
     CPD_TRY(dev_alloc(&d_stats, 5 * sizeof(unsigned long long), st));
     CPD_TRY(cudaMemsetAsync(d_stats, 0, 2 * sizeof(unsigned long long), st));
     CPD_TRY(cudaMemsetAsync(d_stats + 2, 0x7f, 3 * sizeof(unsigned long long), st));
-    // A list that an earlier build left is filled as it is counted.
-    const bool refill = out.idx && out.cap > 0 && !with_mu && !min_spacing;
+    // A list of short rows that an earlier build left is filled as it is
+    // counted.
+    const bool refill = out.idx && out.cap > 0 && out.cap <= kRefillRow && !with_mu && !min_spacing;
     if (refill)
         k_refill<<<blocks_for(npad), kBlock, 0, st>>>(pos, n, npad, begin, g, cell_start, co,
                                                       rsqr, out.count, user_id, out.cap, out.idx,
