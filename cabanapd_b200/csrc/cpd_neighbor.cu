@@ -99,11 +99,11 @@ __global__ void k_cell_index(const double* pos, int64_t n, int64_t npad, Grid g,
     atomicAdd(cell_count + id, 1);
 }
 
-// The particles in cell order: their positions (one plane per component, so
-// that the lanes of a warp, on neighbouring runs, read neighbouring values)
-// and their indices.
+// The particles in cell order: their indices and, for the one-pass fill, their
+// positions (one plane per component, so that the lanes of a warp, on
+// neighbouring runs, read neighbouring values).
 struct CellOrder {
-    const double* pos;  // [3][n]
+    const double* pos;  // [3][n], or null
     const int32_t* index;
     int64_t n;
 };
@@ -115,17 +115,20 @@ __global__ void __launch_bounds__(kBlock)
     if (i >= n) return;
     const int32_t c = cell[i];
     const int32_t slot = cell_start[c] + atomicAdd(cursor + c, 1);
-    for (int d = 0; d < 3; d++) sorted[d * n + slot] = pos[d * npad + i];
+    if (sorted)
+        for (int d = 0; d < 3; d++) sorted[d * n + slot] = pos[d * npad + i];
     index[slot] = (int32_t)i;
 }
 
-// Calls emit(j, dx, dy, dz) for every j != i within the cutoff: walks the (2R + 1)^2
-// lines of cells around particle i in increasing (z, y); the cells of one
-// line are consecutive cell ids, so their particles are one contiguous run
-// of the cell-sorted order. With cells about cutoff / 3 wide, a lattice
+// Calls emit(j, dx, dy, dz) for every j != i within the cutoff: walks the
+// (2R + 1)^2 lines of cells around particle i in increasing (z, y); the cells
+// of one line are consecutive cell ids, so their particles are one contiguous
+// run of the cell-sorted order. With cells about cutoff / 3 wide, a lattice
 // holds about one particle per cell and an x-fastest lattice row is emitted
 // in nearly ascending index order (the row sort then moves little).
-template <typename Emit>
+// SORTED: candidates from the cell-sorted positions (co.pos), the index read of
+// those within the cutoff only; otherwise through their index.
+template <bool SORTED, typename Emit>
 __device__ __forceinline__ void visit_neighbors(const double* __restrict__ pos, int64_t npad,
                                                 const Grid& g, const int32_t* __restrict__ cell_start,
                                                 const CellOrder& co, int64_t i,
@@ -144,13 +147,22 @@ __device__ __forceinline__ void visit_neighbors(const double* __restrict__ pos, 
             const int64_t line = (int64_t)g.nc[0] * (cy + (int64_t)g.nc[1] * cz);
             const int32_t q1 = __ldg(cell_start + line + cx1 + 1);
             for (int32_t q = __ldg(cell_start + line + cx0); q < q1; q++) {
-                const double ddx = __ldg(co.pos + q) - px;
-                const double ddy = __ldg(co.pos + co.n + q) - py;
-                const double ddz = __ldg(co.pos + 2 * co.n + q) - pz;
+                int64_t j = i;
+                if (!SORTED) {
+                    j = __ldg(co.index + q);
+                    if (j == i) continue;
+                }
+                const double ddx = (SORTED ? __ldg(co.pos + q) : pos[j]) - px;
+                const double ddy = (SORTED ? __ldg(co.pos + co.n + q) : pos[npad + j]) - py;
+                const double ddz =
+                    (SORTED ? __ldg(co.pos + 2 * co.n + q) : pos[2 * npad + j]) - pz;
                 const double d2 = ddx * ddx + ddy * ddy + ddz * ddz;
                 if (!(d2 <= rsqr)) continue;
-                const int64_t j = __ldg(co.index + q);
-                if (j != i) emit(j, ddx, ddy, ddz);
+                if (SORTED) {
+                    j = __ldg(co.index + q);
+                    if (j == i) continue;
+                }
+                emit(j, ddx, ddy, ddz);
             }
         }
     }
@@ -172,6 +184,7 @@ __device__ __forceinline__ void row_stats(int32_t cnt, unsigned long long* stats
 // over the accepted pairs (the bit patterns of non-negative doubles order
 // like the values), the lattice spacing the mixed path's stencil needs.
 // stats: [0] the longest row, [1] the sum of the row lengths.
+template <bool SORTED>
 __global__ void __launch_bounds__(kBlock)
     k_count(const double* pos, int64_t n, int64_t npad, int64_t begin, Grid g,
             const int32_t* cell_start, CellOrder co, double rsqr, int32_t* count,
@@ -183,7 +196,7 @@ __global__ void __launch_bounds__(kBlock)
     int32_t cnt = 0;
     if (i < npad) {
         if (i >= begin && i < n)
-            visit_neighbors(pos, npad, g, cell_start, co, i, rsqr,
+            visit_neighbors<SORTED>(pos, npad, g, cell_start, co, i, rsqr,
                             [&](int64_t, double dx, double dy, double dz) {
                                 cnt++;
                                 if (min_out) {
@@ -232,7 +245,7 @@ __global__ void __launch_bounds__(kBlock)
     int32_t cnt = 0;
     if (i < npad) {
         if (i >= begin && i < n) {
-            visit_neighbors(pos, npad, g, cell_start, co, i, rsqr,
+            visit_neighbors<true>(pos, npad, g, cell_start, co, i, rsqr,
                             [&](int64_t j, double, double, double) {
                                 if (cnt < cap) {
                                     // Insert by key from the end of the row.
@@ -258,6 +271,7 @@ __global__ void __launch_bounds__(kBlock)
 // Fill row i and sort it by the caller index of the neighbour. Rows that fit
 // kLocalRow are sorted in a thread-local array; longer rows are sorted in
 // place in the column-major list.
+template <bool SORTED>
 __global__ void __launch_bounds__(kBlock)
     k_fill(const double* pos, int64_t n, int64_t npad, int64_t begin, Grid g,
            const int32_t* cell_start, CellOrder co, double rsqr,
@@ -270,7 +284,7 @@ __global__ void __launch_bounds__(kBlock)
     if (cnt <= kLocalRow) {
         int32_t row[kLocalRow];
         int32_t k = 0;
-        visit_neighbors(pos, npad, g, cell_start, co, i, rsqr,
+        visit_neighbors<SORTED>(pos, npad, g, cell_start, co, i, rsqr,
                         [&](int64_t j, double, double, double) {
                             if (k < kLocalRow) row[k] = (int32_t)j;
                             k++;
@@ -288,7 +302,7 @@ __global__ void __launch_bounds__(kBlock)
         for (int32_t a = 0; a < cnt; a++) idx[(int64_t)a * npad + i] = row[a];
     } else {
         int32_t k = 0;
-        visit_neighbors(pos, npad, g, cell_start, co, i, rsqr,
+        visit_neighbors<SORTED>(pos, npad, g, cell_start, co, i, rsqr,
                         [&](int64_t j, double, double, double) {
                             if (k < max_n) idx[(int64_t)k * npad + i] = (int32_t)j;
                             k++;
@@ -467,29 +481,50 @@ int build_neighbor_list(const double* x, const double* disp, int64_t n, int64_t 
             lo[d] = std::min(lo[d], part[6 * b + d]);
             hi[d] = std::max(hi[d], part[6 * b + 3 + d]);
         }
-    // Cells a little over a third of the cutoff wide (visit radius 3), grown
-    // by doubling while the grid would hold far more cells than particles
-    // (visit radius 2, then 1). The 1e-9 margin keeps cutoff / cell below the
-    // radius, so pairs within the cutoff are at most R cells apart.
-    // Sparse lists (contact: a few neighbours a row) take cells of the cutoff,
-    // visit radius 1: 9 lines of cells per row instead of 49, each a chain of
-    // dependent loads, for about twice the candidates (4.0 M spheres at 3.8
-    // expected neighbours: 4.78 vs 5.14 ms per 20 steps with two rebuilds; at
-    // 7.4: 7.8 vs 8.0; bonds at 114 expect the third: 343 candidates a row
-    // instead of 729).
+    // A list of short rows that an earlier build left is filled as it is
+    // counted.
+    const bool refill = out.idx && out.cap > 0 && out.cap <= kRefillRow && !with_mu && !min_spacing;
+    // Cells a little over a third of the cutoff wide (visit radius 3: 49 lines
+    // of cells and 13 cutoffs cubed of candidates a row) where the grid then
+    // holds few more cells than particles; else cells of the cutoff (9 lines,
+    // 27 cutoffs cubed), or of 4/3, 8/3, ... of it. The 1e-9 margin keeps cutoff
+    // / cell below the radius, so pairs within the cutoff are at most R cells
+    // apart. (Cells of two thirds, which a grid too fine by up to eight times
+    // would allow, mean 25 lines and 37 cutoffs cubed: 1.0 M random points with
+    // mean rows of 24, count and fill, 5.0 ms against 4.0.)
+    // The one-pass fill takes cells of the cutoff first: its walk is short of
+    // loads in flight, and 9 lines are fewer dependent chains (1.0 M lattice
+    // points, rows of 32: 2.23 vs 2.62 ms per step with a rebuild). Where even
+    // those are too fine, either the rows are nearly empty (1.0 M points, mean
+    // rows of 1: 0.51 ms in cells of 4/3, 0.82 of 2) or the box is: then most
+    // lines of cells are looked up for nothing, and cells of 2 are faster (a
+    // shell of 0.5 M points, mean rows of 1.7, 3.4 and 6.8: 1.18, 0.75 and 1.27
+    // ms, 1.86, 1.09 and 1.94 in cells of 4/3). The earlier list's mean row
+    // tells them apart.
     Grid g;
-    double vol = 1.0;
-    for (int d = 0; d < 3; d++) vol *= std::max(hi[d] - lo[d], cutoff);
-    const double expect = 4.18879 * cutoff * cutoff * cutoff * (double)n / vol;
-    double cell = (expect < 16.0 ? cutoff : cutoff / 3.0) * (1.0 + 1e-9);
-    for (;;) {
+    auto fits = [&](double cell) {
         for (int d = 0; d < 3; d++) {
             double span = (hi[d] - lo[d]) / cell;
             g.nc[d] = (int32_t)std::max<int64_t>(1, std::min<int64_t>((int64_t)span + 1, 1 << 20));
         }
-        if ((double)g.nc[0] * g.nc[1] * g.nc[2] <= 4.0 * (double)n + 4096.0) break;
-        cell *= 2.0;
+        return (double)g.nc[0] * g.nc[1] * g.nc[2] <= 4.0 * (double)n + 4096.0;
+    };
+    double cell = cutoff / 3.0 * (1.0 + 1e-9);
+    bool whole = false;  // cells of the cutoff
+    if (refill || !fits(cell)) {
+        cell = cutoff * (1.0 + 1e-9);
+        whole = fits(cell);
+        if (!whole) {
+            const bool hollow = refill && 2 * out.total >= 3 * (n - begin);
+            for (cell *= hollow ? 2.0 : 4.0 / 3.0; !fits(cell);) cell *= 2.0;
+        }
     }
+    // The cell-sorted positions serve the one-pass fill and cells of the cutoff.
+    // Elsewhere the walk is bound by how its lanes' candidates lie in memory, and
+    // a lattice whose order is not x fastest has them side by side in its own
+    // order and apart in the cells' (1.0 M points z fastest, rows of 32, cells of
+    // a third: 2.6 ms per step with a rebuild, 3.6 with sorted positions).
+    const bool by_cell = refill || whole;
     for (int d = 0; d < 3; d++) g.lo[d] = lo[d];
     g.cell = cell;
     g.R = std::max(1, (int32_t)std::ceil(cutoff / cell - 1e-9));
@@ -502,7 +537,7 @@ int build_neighbor_list(const double* x, const double* disp, int64_t n, int64_t 
     CPD_TRY(dev_alloc(&cell_count, sizeof(int32_t) * (ncell + 1), st));
     CPD_TRY(dev_alloc(&cell_start, sizeof(int32_t) * (ncell + 1), st));
     CPD_TRY(dev_alloc(&index, sizeof(int32_t) * n, st));
-    CPD_TRY(dev_alloc(&sorted, sizeof(double) * 3 * n, st));
+    if (by_cell) CPD_TRY(dev_alloc(&sorted, sizeof(double) * 3 * n, st));
     CPD_TRY(cudaMemsetAsync(cell_count, 0, sizeof(int32_t) * (ncell + 1), st));
     k_cell_index<<<blocks_for(n), kBlock, 0, st>>>(pos, n, npad, g, cellid, cell_count);
     launches++;
@@ -529,18 +564,14 @@ int build_neighbor_list(const double* x, const double* disp, int64_t n, int64_t 
     CPD_TRY(dev_alloc(&d_stats, 5 * sizeof(unsigned long long), st));
     CPD_TRY(cudaMemsetAsync(d_stats, 0, 2 * sizeof(unsigned long long), st));
     CPD_TRY(cudaMemsetAsync(d_stats + 2, 0x7f, 3 * sizeof(unsigned long long), st));
-    // A list of short rows that an earlier build left is filled as it is
-    // counted.
-    const bool refill = out.idx && out.cap > 0 && out.cap <= kRefillRow && !with_mu && !min_spacing;
     if (refill)
         k_refill<<<blocks_for(npad), kBlock, 0, st>>>(pos, n, npad, begin, g, cell_start, co,
                                                       rsqr, out.count, user_id, out.cap, out.idx,
                                                       d_stats);
     else
-        k_count<<<blocks_for(npad), kBlock, 0, st>>>(pos, n, npad, begin, g, cell_start, co,
-                                                     rsqr, out.count,
-                                                     min_spacing ? d_stats + 2 : nullptr,
-                                                     d_stats);
+        (by_cell ? k_count<true> : k_count<false>)<<<blocks_for(npad), kBlock, 0, st>>>(
+            pos, n, npad, begin, g, cell_start, co, rsqr, out.count,
+            min_spacing ? d_stats + 2 : nullptr, d_stats);
     launches++;
     unsigned long long hstats[5];
     CPD_TRY(cudaMemcpyAsync(hstats, d_stats, sizeof(hstats), cudaMemcpyDeviceToHost, st));
@@ -573,9 +604,8 @@ int build_neighbor_list(const double* x, const double* disp, int64_t n, int64_t 
     out.nwords = (max_n + 31) / 32;
     tr.mark("alloc", st);
     if (n > begin && !filled) {
-        k_fill<<<blocks_for(n - begin), kBlock, 0, st>>>(pos, n, npad, begin, g, cell_start,
-                                                        co, rsqr, out.count, user_id,
-                                                        max_n, out.idx);
+        (by_cell ? k_fill<true> : k_fill<false>)<<<blocks_for(n - begin), kBlock, 0, st>>>(
+            pos, n, npad, begin, g, cell_start, co, rsqr, out.count, user_id, max_n, out.idx);
         launches++;
     }
     if (with_mu && out.nwords > 0) {
@@ -604,7 +634,7 @@ int build_neighbor_list(const double* x, const double* disp, int64_t n, int64_t 
     CPD_TRY(dev_free(cell_count, st));
     CPD_TRY(dev_free(cell_start, st));
     CPD_TRY(dev_free(index, st));
-    CPD_TRY(dev_free(sorted, st));
+    if (sorted) CPD_TRY(dev_free(sorted, st));
     if (y) CPD_TRY(dev_free(y, st));
     return launches;
 }
