@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(kBlock, 4)
 enum { M_PMB = 0, M_LPS = 1, M_LINEAR_PMB = 2 };
 
 template <int MODEL, int INFL, bool FRACTURE>
-__global__ void __launch_bounds__(kBlock, MODEL == M_LPS ? 4 : 3)
+__global__ void __launch_bounds__(kBlock, 3)
     k_pd_force(ParticleView p, EllView nl, ModelDev md)
 {
     const int64_t i = p.frozen + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -310,7 +310,9 @@ __global__ void __launch_bounds__(kBlock, MODEL == M_LPS ? 4 : 3)
         // series; their breaking and sums stay in row order. Indices are read
         // a pair ahead. (An odd row's last pair holds its last bond twice; the
         // copy adds nothing.) LPS carries two more gathers per bond and is
-        // faster with one bond at a time and a block more per SM.
+        // faster with one bond at a time (box of 1.0 M rows, per step: 2.16 ms
+        // at three blocks of 256 per SM; four, with the spills of 64 registers,
+        // 2.26; two bonds at a time 2.4).
         constexpr int NB = lps ? 1 : 2;
         const BondEnd me{xi0, xi1, xi2, ui0, ui1, ui2};
         int32_t jn[NB];
@@ -434,7 +436,7 @@ __global__ void __launch_bounds__(kBlock, 3)
         for (int k = 0; k < cnt; ++k) {
             if (FRACTURE && (k & 31) == 0) word = nl.mu[(int64_t)(k >> 5) * np + i];
             const int64_t j = jn;
-        if (k + 1 < cnt) jn = __ldg(nl.idx + (int64_t)(k + 1) * np + i);
+            if (k + 1 < cnt) jn = __ldg(nl.idx + (int64_t)(k + 1) * np + i);
             const double vol_j = __ldg(p.vol + j);
             double s, xi;
             Divisor X;
@@ -1028,9 +1030,11 @@ int launch_pd_force(const ParticleView& p, const EllView& nl, const Model& md,
 {
     const int64_t rows = p.n - p.frozen;
     if (rows <= 0) return 0;
-    // Small bodies take smaller blocks, so that the blocks spread evenly over
-    // the SMs (79 thousand rows: 106 vs 112 us per step).
-    const int block = rows < (int64_t)148 * 12 * kBlock ? kBlock / 2 : kBlock;
+    // Blocks of half the size spread more evenly over the SMs (plates, per step
+    // in blocks of 128 / 256: 20 thousand rows 62 / 65 us, 80: 102 / 107, 200:
+    // 201 / 209, 440: 419 / 427, 800: 762 / 770; an LPS box of 2.0 M: 4.52 / 4.54
+    // ms).
+    constexpr int block = kBlock / 2;
     const int g = (int)((rows + block - 1) / block);
     const ModelDev d = to_dev(md);
     CPD_PD_DISPATCH(k_pd_force, g, block, p, nl, d);
