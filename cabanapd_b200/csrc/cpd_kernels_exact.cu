@@ -49,10 +49,16 @@ ModelDev to_dev(const Model& m)
 //         (P. W. Markstein, IBM J. Res. Dev. 34, 1990).
 // Next to a midpoint, outside the middle of the exponent range (where a
 // residual could round) and for a divisor that ends in ones the IEEE
-// operations are taken, so every result is the IEEE one. Issue-bound (68%;
-// FP64 pipe 56%): 189 instructions per bond; on a 1.0 M-particle plate 0.94
-// instead of 1.10 ms per force pass, on 79 thousand rows, where the chains'
-// latency counts, 1.07 instead of 1.37 ms per ten steps and the totals.
+// operations are taken, so every result is the IEEE one, but for the sign of a
+// zero: the quotient of -0 is +0 here. The callers add their quotients to sums
+// that start at +0, where neither zero changes anything. (The root's test is by
+// the unit above a power of two; below one only the double next under an even
+// power has its root next to a midpoint, and every y within an ulp of its
+// reciprocal root gives a sum on the upper side, where the test sees it.)
+// Issue-bound (68%; FP64 pipe 56%): 189 instructions per bond; on a 1.0
+// M-particle plate 0.94 instead of 1.10 ms per force pass, on 79 thousand rows,
+// where the chains' latency counts, 1.07 instead of 1.37 ms per ten steps and
+// the totals.
 __device__ __forceinline__ bool mid_square(double v)  // v in [2^-900, 2^900)
 {
     return (uint32_t)(__double2hiint(v) - 0x07b00000) < 0x70800000u;
