@@ -47,18 +47,17 @@ ModelDev to_dev(const Model& m)
 //   1 / b two Newton steps on y, correctly rounded unless b's significand is
 //         all ones; quotients by two corrections with exact remainders
 //         (P. W. Markstein, IBM J. Res. Dev. 34, 1990).
-// Next to a midpoint, outside the middle of the exponent range (where a
-// residual could round) and for a divisor that ends in ones the IEEE
-// operations are taken, so every result is the IEEE one, but for the sign of a
+// Next to a midpoint and for a divisor that ends in ones settle() decides, and
+// outside the middle of the exponent range (where a residual could round) the
+// IEEE operations are taken, so every result is the IEEE one, but for the sign of a
 // zero: the quotient of -0 is +0 here. The callers add their quotients to sums
 // that start at +0, where neither zero changes anything. (The root's test is by
 // the unit above a power of two; below one only the double next under an even
 // power has its root next to a midpoint, and every y within an ulp of its
 // reciprocal root gives a sum on the upper side, where the test sees it.)
-// Issue-bound (68%; FP64 pipe 56%): 189 instructions per bond; on a 1.0
-// M-particle plate 0.94 instead of 1.10 ms per force pass, on 79 thousand rows,
-// where the chains' latency counts, 1.07 instead of 1.37 ms per ten steps and
-// the totals.
+// Issue-bound (68%; FP64 pipe 56%). Plates of 1.0 M and 80 thousand rows: 924
+// and 100 us per step, 1095 and 132 with IEEE operations throughout; LPS boxes
+// of the same sizes 1947 and 160, 2520 and 197.
 __device__ __forceinline__ bool mid_square(double v)  // v in [2^-900, 2^900)
 {
     return (uint32_t)(__double2hiint(v) - 0x07b00000) < 0x70800000u;
@@ -104,6 +103,32 @@ __device__ __forceinline__ double root(double a, double y, bool& ok)
     ok = ok && (__double2hiint(left) & 0x7fffffff) < half - 1;
     return r;
 }
+// Where root() or divisor() could not tell: r, next to RN(sqrt(a)), to the
+// rounded root by the signs of a less the products with its neighbours (the
+// Tuckerman test), and its reciprocal; all ones are 2^e (1 - 2^-53), whose
+// reciprocal rounds to 2^-e (1 + 2^-52). Lengths just below a power of two are
+// no rarity: on a lattice of 24, 48 or 96 cells to the unit three spacings are
+// one, six bonds of every row (cubes of 24, 48 and 96 cells: 71, 137 and 855 us
+// per step, 83, 153 and 939 with the IEEE root and quotients for both lengths).
+__device__ __forceinline__ void settle(double a, double& r, Divisor& d)
+{
+    if (!mid_square(a)) {
+        r = sqrt(a);
+        d = Divisor{r, 0.0, false};
+        return;
+    }
+    const double up = __longlong_as_double(__double_as_longlong(r) + 1);
+    const double down = __longlong_as_double(__double_as_longlong(r) - 1);
+    if (fma(-r, up, a) > 0.0)
+        r = up;
+    else if (fma(-r, down, a) <= 0.0)
+        r = down;
+    const int32_t high = __double2hiint(r);
+    d = divisor(r, d.y, true);
+    if (__double2loint(r) == -1 && (high & 0xfffff) == 0xfffff)
+        d.y = __hiloint2double((2045 - (high >> 20)) << 20, 1);
+    d.fast = true;
+}
 
 // CabanaPD_Force.hpp:74-93 getDistance for the pair (i, j); particle i's
 // position and displacement are already in registers. R: r as a divisor; X:
@@ -134,20 +159,18 @@ __device__ __forceinline__ void bond_geometry(const BondEnd& a, const BondEnd& b
     g.rz = g.xz + eta_w;
     const double r2 = g.rx * g.rx + g.ry * g.ry + g.rz * g.rz;
     const double x2 = g.xx * g.xx + g.xy * g.xy + g.xz * g.xz;
-    bool ok = mid_square(r2) && mid_square(x2);
+    bool ok_r = mid_square(r2), ok_x = mid_square(x2);
     const double yr = rsqrt(r2), yx = rsqrt(x2);
-    g.r = root(r2, yr, ok);
-    g.xi = root(x2, yx, ok);
-    g.X = divisor(g.xi, yx, ok);
-    g.R = divisor(g.r, yr, ok);
+    g.r = root(r2, yr, ok_r);
+    g.xi = root(x2, yx, ok_x);
+    g.X = divisor(g.xi, yx, ok_x);
+    g.R = divisor(g.r, yr, ok_r);
     // (r - xi is exact or far above the range where a remainder could round.)
     g.s = quotient(g.r - g.xi, g.X);
-    if (!g.X.fast) {
-        g.r = sqrt(r2);
-        g.xi = sqrt(x2);
-        g.s = (g.r - g.xi) / g.xi;
-        g.R = Divisor{g.r, 0.0, false};
-        g.X = Divisor{g.xi, 0.0, false};
+    if (!(g.X.fast && g.R.fast)) {
+        if (!g.R.fast) settle(r2, g.r, g.R);
+        if (!g.X.fast) settle(x2, g.xi, g.X);
+        g.s = divide(g.r - g.xi, g.X);
     }
 }
 // The form the passes without a force take.
@@ -316,9 +339,10 @@ __global__ void __launch_bounds__(kBlock, 3)
         // series; their breaking and sums stay in row order. Indices are read
         // a pair ahead. (An odd row's last pair holds its last bond twice; the
         // copy adds nothing.) LPS carries two more gathers per bond and is
-        // faster with one bond at a time (box of 1.0 M rows, per step: 2.16 ms
-        // at three blocks of 256 per SM; four, with the spills of 64 registers,
-        // 2.26; two bonds at a time 2.4).
+        // faster with one bond at a time (box of 1.0 M rows: 2.26 against 2.4 ms
+        // per step) and at three blocks of 256 per SM (2.16; four: 2.26, with
+        // the spills of 64 registers). Whether a bond breaks is decided beside
+        // its force, so that its lengths need not be kept.
         constexpr int NB = lps ? 1 : 2;
         const BondEnd me{xi0, xi1, xi2, ui0, ui1, ui2};
         int32_t jn[NB];
@@ -331,9 +355,8 @@ __global__ void __launch_bounds__(kBlock, 3)
                 dirty = false;
                 word = nl.mu[(int64_t)(k >> 5) * np + i];
             }
-            Geometry g[NB];
             double qx[NB], qy[NB], qz[NB];
-            bool safe[NB];
+            bool breaks[NB];
 #pragma unroll
             for (int b = 0; b < NB; ++b) {
                 const int64_t j = jn[b];
@@ -341,26 +364,29 @@ __global__ void __launch_bounds__(kBlock, 3)
                 const double vol_j = __ldg(p.vol + j);
                 // LPS tests nofail(i) twice (force/CabanaPD_LPS.hpp:417-418),
                 // PMB nofail(i) and nofail(j).
-                safe[b] = FRACTURE && (nofail_i || (!lps && __ldg(p.nofail + j) != 0));
-                bond_geometry(me, bond_end(p.x, p.u, np, j), g[b]);
+                const bool safe = FRACTURE && (nofail_i || (!lps && __ldg(p.nofail + j) != 0));
+                Geometry g;
+                bond_geometry(me, bond_end(p.x, p.u, np, j), g);
+                // CabanaPD_ForceModels.hpp:123-128.
+                breaks[b] = FRACTURE && g.r * g.r >= md.bond_break_coeff * g.xi * g.xi && !safe;
                 double coeff;
                 if (lps) {
                     const double a_j = __ldg(p.lps_a + j), b_j = __ldg(p.lps_b + j);
-                    coeff = (a_i + a_j + g[b].s * (b_i + b_j)) * influence<INFL>(g[b].X) *
-                            g[b].xi * vol_j;
+                    coeff = (a_i + a_j + g.s * (b_i + b_j)) * influence<INFL>(g.X) *
+                            g.xi * vol_j;
                 } else {
-                    coeff = md.c * g[b].s * vol_j;
+                    coeff = md.c * g.s * vol_j;
                 }
-                const double px = coeff * g[b].rx, py = coeff * g[b].ry, pz = coeff * g[b].rz;
-                qx[b] = quotient(px, g[b].R);
-                qy[b] = quotient(py, g[b].R);
-                qz[b] = quotient(pz, g[b].R);
-                if (!(g[b].R.fast &&
+                const double px = coeff * g.rx, py = coeff * g.ry, pz = coeff * g.rz;
+                qx[b] = quotient(px, g.R);
+                qy[b] = quotient(py, g.R);
+                qz[b] = quotient(pz, g.R);
+                if (!(g.R.fast &&
                       max(max(value_range(px), value_range(py)), value_range(pz)) < 0x7d000000u) &&
-                    !(g[b].R.fast && mid_value(px) && mid_value(py) && mid_value(pz))) {
-                    qx[b] = px / g[b].r;
-                    qy[b] = py / g[b].r;
-                    qz[b] = pz / g[b].r;
+                    !(g.R.fast && mid_value(px) && mid_value(py) && mid_value(pz))) {
+                    qx[b] = px / g.r;
+                    qy[b] = py / g.r;
+                    qz[b] = pz / g.r;
                 }
             }
 #pragma unroll
@@ -368,11 +394,8 @@ __global__ void __launch_bounds__(kBlock, 3)
                 if (k + b >= cnt) continue;
                 bool intact = true;
                 if (FRACTURE) {
-                    // CabanaPD_ForceModels.hpp:123-128.
-                    const bool critical =
-                        g[b].r * g[b].r >= md.bond_break_coeff * g[b].xi * g[b].xi;
                     const uint32_t bit = 1u << ((k + b) & 31);
-                    if (critical && !safe[b]) {
+                    if (breaks[b]) {
                         if (word & bit) {
                             word &= ~bit;
                             dirty = true;
