@@ -323,12 +323,15 @@ __global__ void __launch_bounds__(kBlock, 3)
     bool dirty = false;
     const int32_t* __restrict__ const row = nl.idx + i;
     if (linear) {
+        int32_t jn = cnt > 0 ? __ldg(row) : 0;  // (read one bond ahead)
         for (int k = 0; k < cnt; ++k) {
-            const int64_t j = __ldg(row + (int64_t)k * np);
+            const int64_t j = jn;
+            if (k + 1 < cnt) jn = __ldg(row + (int64_t)(k + 1) * np);
+            const double vol_j = __ldg(p.vol + j);
             double xi, ls, xx, xy, xz;
             bond_linearized(p.x, p.u, np, j, xi0, xi1, xi2, ui0, ui1, ui2, xi, ls,
                             xx, xy, xz);
-            const double coeff = md.c * ls * __ldg(p.vol + j);
+            const double coeff = md.c * ls * vol_j;
             fx += coeff * xx / xi;
             fy += coeff * xy / xi;
             fz += coeff * xz / xi;
