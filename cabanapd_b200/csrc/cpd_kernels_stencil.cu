@@ -66,11 +66,10 @@ inline int blocks_for(int64_t rows) { return (int)((rows + kBlock - 1) / kBlock)
 //   FP32 15 / 19, 15 / 20, 27 / 31, 27 / 31, 40 / 44, 41 / 45 us, and at 238
 //   (7/8) 58 / 58: share 0.875;
 // and between, where the ratio is one (43 to 74, 125 and 149 thousand), FP64
-// 25 / 23, 44 / 41, FP32 20 / 19, 39 / 31 us. The four launches of the wide
-// table gain from whole blocks sooner (20 thousand rows 72 / 83 us, 80 thousand,
-// ratio 3/4, 131 / 125): share 0.6.
+// 25 / 23, 44 / 41, FP32 20 / 19, 39 / 31 us. (The wide table's launches: 81 and
+// 88 thousand rows, ratio 3/4, 117 / 126 and 116 / 127 us.)
 constexpr int kWalkBlock = 512, kSmallWalkBlock = 256;
-constexpr double kShare64 = 0.8, kShare64Wide = 0.6, kShare32 = 0.875;
+constexpr double kShare64 = 0.8, kShare32 = 0.875;
 inline int walk_blocks(int64_t warps, int block)
 {
     return (int)((warps + block / 32 - 1) / (block / 32));
@@ -831,7 +830,7 @@ int launch_pd_force_stencil64(const ParticleView& p, const EllView& nl, const Mo
     int launched = 0;
     if (m.nstencil > 0) {
         const StencilRows sr{m.warp_kind, m.pmask, m.stencil_list, m.nstencil};
-        const int block = walk_block(m.nstencil, m.st64w ? kShare64Wide : kShare64);
+        const int block = walk_block(m.nstencil, kShare64);
         const int g = walk_blocks(m.nstencil, block);
         const bool uniform = m.vol_sums != nullptr;
         if (m.st64w) {
