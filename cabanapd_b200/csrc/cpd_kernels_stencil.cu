@@ -185,6 +185,24 @@ __device__ __forceinline__ bool exact_bond(const ParticleView& p, int64_t i, int
     return false;
 }
 
+// A gather record in one 32-byte load (two 16-byte loads touch every line of a
+// warp's records twice: 2.75 vs 2.51 ms per step on the 11.52 M plate). ORDERED
+// (the energy forms): loads stay in the order of the walk; left free, more
+// records are brought ahead than 64 registers hold beside the energy terms
+// (elastic form: 660 bytes of spill stores, 44 in order; a step with the totals
+// of 593 thousand rows 266 and 252 us). The steps themselves are faster free
+// (2.51 vs 2.56 ms).
+template <bool ORDERED>
+__device__ __forceinline__ Record64 load_record(const char* p)
+{
+    if (!ORDERED) return *reinterpret_cast<const Record64*>(p);
+    Record64 v;
+    asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
+                 : "l"(p));
+    return v;
+}
+
 // One bond of the unrolled table walk: entry e of row i, gather record uj.
 // Adds F r_vec to f when the bond is present and intact (bit on) and num is
 // inside the entry's window; a present bond outside it is deferred (pend).
@@ -367,15 +385,13 @@ __global__ void __launch_bounds__(kWalkBlock, 2)
     // Fully unrolled, every entry of the range for every row: an absent entry
     // (no bit in ew) reads the record at i + delta_k (a neighbour, or a zero
     // guard record) and adds nothing, which costs less than a branch per
-    // entry. Entries past ntab are zero-filled and add nothing either. The
-    // record is one 32-byte load (two 16-byte loads touch every line of a
-    // warp's records twice: 2.75 vs 2.51 ms per step on the 11.52 M plate).
+    // entry. Entries past ntab are zero-filled and add nothing either.
 #pragma unroll
     for (int k = K0; k < K1; ++k) {
         const int w = k >> 5;
         const uint32_t bit = 1u << (k & 31);
         const StencilEntry64& e = st.e[k];
-        const Record64 uj = *reinterpret_cast<const Record64*>(rb + e.boff);
+        const Record64 uj = load_record<ENERGY>(rb + e.boff);
         stencil_bond64<UNIFORM, NP, ENERGY>(e, st.h, uj, ui, (ew[w] & bit) != 0u, bit, pend[w],
                                             fx, fy, fz, st.sh, ENERGY ? st.kw[k] : 0.0, &wsum);
     }
